@@ -181,7 +181,7 @@ _DS_MAX_BYTES = int(os.environ.get("GT_ATTN_DS_MAX_MB", "4096")) << 20
 
 def ds_buffer(blk, h, dtype, device):
     """The hand-off buffer of a block, or ``None`` when the passes run independently."""
-    if not _DS_ON or dtype != torch.bfloat16 or blk.num_edges == 0 or blk.num_edges * h * 4 > _DS_MAX_BYTES:
+    if not _DS_ON or blk.num_edges == 0 or blk.num_edges * h * 4 > _DS_MAX_BYTES:
         return None
     return torch.empty(blk.num_edges, h, dtype=torch.float32, device=device)
 

@@ -7,15 +7,11 @@ a products-like 612K x 612K tile and a dense-ish Reddit-like tile.  Options:
   * operand type: bf16 or fp32 Q / K / V (fp32 takes the register-pipelined kernels, bf16 the cp.async ring kernels);
   * head layout at 256 channels: 8 x 32 (compile-time specialised instance), 4 x 64 and 16 x 16 (generic instance);
   * hub-row segment length (``seg_edges``): rows and columns longer than this are cut into segments merged by a second kernel;
-  * ``--no_ring``: re-run the bf16 cases in a child process with ``GT_ATTN_ASYNC=0`` (register-pipelined kernels for bf16).
 
-    python -m gt_b200.bench.bench_kernel_opts [--blocks arxiv tile24] [--no_ring]
+    python -m gt_b200.bench.bench_kernel_opts [--blocks arxiv tile24]
 """
 import argparse
 import json
-import os
-import subprocess
-import sys
 
 import torch
 
@@ -59,11 +55,9 @@ def main(argv=None):
     ap.add_argument("--dtypes", nargs="+", default=["bf16", "fp32"])
     ap.add_argument("--seg_edges", type=int, nargs="+", default=[0], help="0 = the backend's default segment length")
     ap.add_argument("--iters", type=int, default=5)
-    ap.add_argument("--no_ring", action="store_true", help="also run the bf16 cases with GT_ATTN_ASYNC=0 in a child process")
     args = ap.parse_args(argv)
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
-    ring = os.environ.get("GT_ATTN_ASYNC", "1") != "0"
     out = []
     for name in args.blocks:
         n_rows, n_cols, edges = BLOCKS[name]
@@ -74,15 +68,10 @@ def main(argv=None):
                 for seg in args.seg_edges:
                     fwd, bwd = run_case(blk, n_rows, n_cols, h, d, torch.bfloat16 if dt == "bf16" else torch.float32, seg, dev, args.iters)
                     row = dict(block=name, rows=n_rows, cols=n_cols, edges=edges, layout=lay, dtype=dt, seg_edges=seg or "default",
-                               ring=bool(ring and dt == "bf16"), fwd_ms=fwd, bwd_ms=bwd, fwd_ns_per_edge=fwd * 1e6 / edges,
+                               ring=dt == "bf16", fwd_ms=fwd, bwd_ms=bwd, fwd_ns_per_edge=fwd * 1e6 / edges,
                                bwd_ns_per_edge=bwd * 1e6 / edges)
                     out.append(row)
                     print("OPTS " + json.dumps(row), flush=True)
-    if args.no_ring and ring:
-        env = dict(os.environ, GT_ATTN_ASYNC="0")
-        cmd = [sys.executable, "-m", "gt_b200.bench.bench_kernel_opts", "--blocks", *args.blocks, "--layouts", *args.layouts,
-               "--dtypes", "bf16", "--iters", str(args.iters), "--seg_edges", *[str(s) for s in args.seg_edges]]
-        subprocess.run(cmd, env=env, check=True)
     return out
 
 

@@ -10,7 +10,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(ROOT, "csrc")
 BUILD = os.path.join(ROOT, "_ext")
 NAME = "gt_b200_native"
-CU = ["attn.cu", "attn_tile.cu", "spmm.cu", "rowops.cu", "gemm.cu", "p2p.cu"]
+CU = ["attn.cu", "attn_edge_fwd.cu", "attn_edge_col.cu", "attn_edge_row.cu", "attn_tile.cu", "spmm.cu", "rowops.cu", "gemm.cu", "p2p.cu"]
 
 
 def sources():

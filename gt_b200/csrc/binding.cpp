@@ -76,6 +76,7 @@ void attn_fwd(Tensor q, OptT k, OptT v, Tensor idx, OptT etype, OptT gate, OptT 
         for (int i = 0; i < a.push_n; ++i) a.push_slot[i] = reinterpret_cast<void*>(push_ptrs[i]);
         a.push_rows = (int)push_rows; a.push_ld = push_ld; a.push_l_off = (int)push_l_off;
     }
+    a.c.n_src = k.has_value() ? k->size(0) : 0;
     a.q = q.data_ptr();
     a.k = k.has_value() ? k->data_ptr() : nullptr;
     a.v = v.has_value() ? v->data_ptr() : nullptr;
@@ -134,7 +135,7 @@ void attn_bwd_row(Tensor q, Tensor k, Tensor v, Tensor row_vec, Tensor stat, Ten
     if (a.ds_in) TORCH_CHECK(ds_in->scalar_type() == torch::kFloat32 && ds_in->is_contiguous() && ds_in->numel() == idx.numel() * H,
                              "ds_in must be a contiguous fp32 [E, H] tensor");
     a.c = make_common(q, H, D, idx, etype, gate, bias, plan, scratch, score, norm, scale, lo, hi);
-    a.c.ldq = ldq; a.c.ldk = ldk; a.c.ldr = ldr; a.c.ldo = ldo;
+    a.c.n_src = k.size(0); a.c.ldq = ldq; a.c.ldk = ldk; a.c.ldr = ldr; a.c.ldo = ldo;
     TORCH_CHECK(ldq % 8 == 0 && ldk % 8 == 0 && ldr % 8 == 0 && ldo % 8 == 0, "row strides must be multiples of 8 elements");
     TORCH_CHECK(row_vec.scalar_type() == q.scalar_type(), "row_vec must have the dtype of q");
     a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.row_vec = row_vec.data_ptr();
@@ -157,7 +158,7 @@ void attn_bwd_col(Tensor q, Tensor k, Tensor v, Tensor row_vec, Tensor stat, Ten
     if (a.ds_out) TORCH_CHECK(a.pos != nullptr && ds_out->is_contiguous() && ds_out->numel() == rowidx.numel() * H && pos->numel() == rowidx.numel(),
                               "ds_out must be a contiguous fp32 [E, H] tensor and pos the CSR position of every CSC entry");
     a.c = make_common(q, H, D, rowidx, etype_t, gate, bias, plan, scratch, score, norm, scale, lo, hi);
-    a.c.ldq = ldq; a.c.ldk = ldk; a.c.ldr = ldr; a.c.ldo = ldo;
+    a.c.n_src = q.size(0); a.c.ldq = ldq; a.c.ldk = ldk; a.c.ldr = ldr; a.c.ldo = ldo;
     TORCH_CHECK(ldq % 8 == 0 && ldk % 8 == 0 && ldr % 8 == 0 && ldo % 8 == 0, "row strides must be multiples of 8 elements");
     a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.row_vec = row_vec.data_ptr();
     a.stat = reinterpret_cast<const float4*>(stat.data_ptr<float>());
@@ -178,8 +179,6 @@ std::vector<std::tuple<std::string, int64_t, int64_t, int64_t, int64_t, int64_t>
         out.emplace_back(std::string(k.name), k.regs, k.local_bytes, k.static_smem, k.dyn_smem, k.blocks_per_sm);
     return out;
 }
-
-int64_t attn_status() { return gt::attn_status(); }
 
 bool attn_shape_supported(int64_t H, int64_t D, int64_t T) { return gt::attn_shape_supported((int)H, (int)D, (int)T); }
 
@@ -687,7 +686,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("signal_peers", &signal_peers);
     m.def("wait_flags", &wait_flags);
     m.def("group_barrier", &group_barrier);
-    m.def("attn_status", &attn_status);
     m.def("attn_tile_fwd", &attn_tile_fwd);
     m.def("channel_signal", &channel_signal);
     m.def("sum_payload", &sum_payload);

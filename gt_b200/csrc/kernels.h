@@ -37,6 +37,7 @@ struct AttnCommon {
     // row strides in elements, 0 = dense rows of H*D: q (and the q-side of the passes), k / v, row_vec, and the gradient
     // outputs (dq of the row pass, dk / dv of the column pass).  Operands may be column slices of wider matrices.
     long long ldq, ldk, ldr, ldo;
+    long long n_src;        // rows of the gathered operand (k / v; q in the column pass)
 };
 
 struct AttnFwdArgs {
@@ -59,6 +60,10 @@ struct AttnFwdArgs {
     int push_rows;          // rows per owner
     long long push_ld;      // bf16 elements per payload row
     int push_l_off;         // column of l inside the payload row (multiple of 8)
+    // nullable: normalised output [n_rows, H*D] in the operand type, acc / l (softmax) or acc / (l + eps); acc is then unused and
+    // l / m are dense [n_rows, H]
+    void* o;
+    float eps;
 };
 
 struct AttnBwdRowArgs {
@@ -116,7 +121,6 @@ bool attn_tile_supported(int H, int D, int T);
 int attn_tile_fwd(const AttnTileArgs& a, const void* q, const void* k, const void* v, long long ldq, long long ldk, cudaStream_t s);
 struct KernelInfo { const char* name; int regs; int local_bytes; int static_smem; int dyn_smem; int blocks_per_sm; };
 std::vector<KernelInfo> attn_kernel_info();            // compiled resources of the main attention kernel instances
-int attn_status();                                     // nonzero once after a bounded copy wait of an attention kernel expired (synchronises)
 int attn_bwd_row_blocks(int n_seg);                    // grid size attn_bwd_row will use for n_seg segments
 // sum of per-block partials: out[i] = sum_b part[b, i]
 void reduce_partials(const float* part, int n_blocks, int width, float* out, cudaStream_t s, int accumulate = 0);   // accumulate: out += sum
