@@ -108,10 +108,26 @@ def attn_fwd_partial(q, k, v, blk: BlockCSR, gate=None, bias=None, *, score="dot
         scratch = torch.empty(plan.num_slots, (h * d + 2 * h + 3) // 4 * 4, dtype=torch.float32, device=q.device) if plan.num_slots else None
         native.ext().attn_fwd(q.contiguous(), k.contiguous() if k is not None else None, v.contiguous() if v is not None else None,
                               blk.col, blk.etype, g, b, _plan_list(plan), None, acc, l, m, scratch, h, d, sc, nm, scale, lo, hi,
-                              h * d, h, False, k_peers, v_peers, int(rows_per_peer), 0, 0, [], 0, 0, 0)
+                              h * d, h, False, k_peers, v_peers, int(rows_per_peer), 0, 0, [], 0, 0, 0, None, 0.0)
     if tiles is not None:
         attn_tile_accumulate(q, k, v, tiles, b, acc, l, m, score=score, norm=norm, clamp=(lo, hi), scale=scale)
     return acc, l, m
+
+
+def _attn_fwd_normalized(q, k, v, blk, gate, bias, score, norm, clamp, eps, scale, seg_edges=SEG_EDGES):
+    """``(o, l, m)`` with ``o`` normalised in the kernels' epilogue and stored in the operand type: the fp32 partials of the generic
+    entry point (twice the bytes of ``o``, written, read back and divided) do not exist.  ``m`` is ``None`` for clamp-exp."""
+    n, h, d = q.shape
+    sc, nm, scale, lo, hi = _cfg(q, score, norm, clamp, scale)
+    g, b = _tables(gate, bias, score)
+    plan = blk.row_plan(seg_edges)
+    o = torch.empty(n, h, d, dtype=q.dtype, device=q.device)
+    l = torch.empty(n, h, dtype=torch.float32, device=q.device)
+    m = torch.empty(n, h, dtype=torch.float32, device=q.device) if norm == "softmax" else None
+    scratch = torch.empty(plan.num_slots, (h * d + 2 * h + 3) // 4 * 4, dtype=torch.float32, device=q.device) if plan.num_slots else None
+    native.ext().attn_fwd(q.contiguous(), k.contiguous(), v.contiguous(), blk.col, blk.etype, g, b, _plan_list(plan), None, l, l, m, scratch,
+                          h, d, sc, nm, scale, lo, hi, h * d, h, False, None, None, 0, 0, 0, [], 0, 0, 0, o, float(eps))
+    return o, l, m
 
 
 def _tile_plan_for(q, k, blk, bias, score, k_peers=None):
@@ -160,7 +176,8 @@ def attn_fwd_partial_accum(q, k, v, blk: BlockCSR, gate, bias, packed, hd, *, sc
     qc = q.reshape(n, hd)[rows.long()].contiguous()
     stride = packed.stride(0)
     native.ext().attn_fwd(qc, k.contiguous(), v.contiguous(), blk.col, blk.etype, g, b, _plan_list(plan), rows,
-                          packed, packed[:, hd:], None, scratch, h, d, sc, nm, scale, lo, hi, stride, stride, True, None, None, 0, 0, 0, [], 0, 0, 0)
+                          packed, packed[:, hd:], None, scratch, h, d, sc, nm, scale, lo, hi, stride, stride, True, None, None, 0, 0, 0, [], 0, 0, 0,
+                          None, 0.0)
 
 
 def normalize(acc, l, norm, eps=1e-6, dtype=None):
@@ -279,10 +296,15 @@ def attn_bwd(q, k, v, blk: BlockCSR, gate, bias, o, l, m, do, *, score="dot", no
         f = lambda t: t.float() if t is not None else None          # noqa: E731
         return _bt.attn_bwd(f(q), f(k), f(v), blk, f(gate), f(bias), f(o), f(l), f(m), f(do), score=score, norm=norm, clamp=clamp,
                             eps=eps, scale=scale)
+    if do.shape == o.shape and do.dtype == o.dtype and l.dtype == torch.float32 and (m is None or m.dtype == torch.float32):
+        stat = torch.empty(*l.shape, 4, dtype=torch.float32, device=l.device)
+        native.ext().attn_bwd_stat(do.contiguous(), o.contiguous(), l.contiguous(), m.contiguous() if m is not None else None, stat,
+                                   norm == "softmax", float(eps))
+        return _bwd(q, k, v, blk, gate, bias, do, stat, score, norm, clamp, scale, seg_edges)
     dd = (do.float() * o.float()).sum(-1)
     l = l.float()
     inv = 1.0 / torch.where(l > 0, l, torch.ones_like(l)) if norm == "softmax" else 1.0 / (l + eps)
-    stat = _pack_stat(m, -dd, inv)
+    stat = _pack_stat(m if m is not None else torch.zeros_like(l), -dd, inv)
     return _bwd(q, k, v, blk, gate, bias, do.reshape(q.shape), stat, score, norm, clamp, scale, seg_edges)
 
 
@@ -290,8 +312,11 @@ class _MaskedSparseAttentionCuda(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, gate, bias, blk, cfg):
         score, norm, clamp, eps, scale = cfg
-        acc, l, m = attn_fwd_partial(q, k, v, blk, gate, bias, score=score, norm=norm, clamp=clamp, scale=scale)
-        o = normalize(acc, l, norm, eps).to(q.dtype)
+        if _supported(q, gate, bias) and q.dim() == 3 and _tile_plan_for(q, k, blk, bias, score) is None:
+            o, l, m = _attn_fwd_normalized(q, k, v, blk, gate, bias, score, norm, clamp, eps, scale)
+        else:
+            acc, l, m = attn_fwd_partial(q, k, v, blk, gate, bias, score=score, norm=norm, clamp=clamp, scale=scale)
+            o = normalize(acc, l, norm, eps).to(q.dtype)
         ctx.blk, ctx.cfg = blk, cfg
         ctx.save_for_backward(q, k, v, gate, bias, o, l, m)
         return o

@@ -790,6 +790,31 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, (CPL == 1 ? 5 : 2)) attn_
     }
 }
 
+// Row statistics of the normalised backward.  D / 8 lanes read a head's dO and o once (2 x 87 MB for 169 K nodes x 256 bf16): bound by
+// that traffic.  As tensor operations (two casts, product, sum, reciprocal, stack) it took 0.70 ms of a 2.33 ms forward + backward.
+template <typename T>
+__global__ void attn_bwd_stat_kernel(const T* __restrict__ dout, const T* __restrict__ o, const float* __restrict__ l, const float* __restrict__ m,
+                                     float4* __restrict__ stat, long long chunks, int lph, int softmax, float eps) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long end = (chunks + 31) / 32 * 32;                 // whole warps take part in the shuffles
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < end; i += stride) {
+        float d = 0.f;
+        if (i < chunks) {
+            float a[8], b[8];
+            Vec8<T>::load_nc(dout + i * 8, a);
+            Vec8<T>::load_nc(o + i * 8, b);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) d = fmaf(a[x], b[x], d);
+        }
+        d = head_sum(d, lph);
+        if (i < chunks && i % lph == 0) {
+            const long long r = i / lph;
+            const float lv = l[r];
+            stat[r] = make_float4(m ? m[r] : 0.f, -d, softmax ? 1.f / (lv > 0.f ? lv : 1.f) : 1.f / (lv + eps), 0.f);
+        }
+    }
+}
+
 // out[i] = sum_b part[b, i]: a block owns 32 columns, its 8 thread rows stride over the partial blocks (coalesced
 // 128-byte reads), the 8 sums are folded through shared memory in a fixed order (deterministic)
 __global__ void reduce_partials_kernel(const float* part, int n_blocks, int width, float* out, int accumulate) {
@@ -937,6 +962,19 @@ void attn_bwd_col(const AttnBwdColArgs& a, cudaStream_t s) {
         if (c.dtype == DT_BF16) sum(static_cast<__nv_bfloat16*>(a.dk), static_cast<__nv_bfloat16*>(a.dv));
         else sum(static_cast<float*>(a.dk), static_cast<float*>(a.dv));
     }
+}
+
+void attn_bwd_stat(int dtype, const void* dout, const void* o, const float* l, const float* m, void* stat, long long rows, int D, bool softmax, float eps,
+                   cudaStream_t s) {
+    if (rows <= 0) return;
+    const long long chunks = rows * (D / 8);
+    const int blocks = (int)std::min<long long>((chunks + 255) / 256, 148 * 16);
+    if (dtype == DT_BF16)
+        attn_bwd_stat_kernel<<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), l, m,
+                                                    static_cast<float4*>(stat), chunks, D / 8, softmax, eps);
+    else
+        attn_bwd_stat_kernel<<<blocks, 256, 0, s>>>(static_cast<const float*>(dout), static_cast<const float*>(o), l, m, static_cast<float4*>(stat), chunks,
+                                                    D / 8, softmax, eps);
 }
 
 namespace {

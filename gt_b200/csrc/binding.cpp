@@ -61,7 +61,7 @@ gt::AttnCommon make_common(const Tensor& q, int64_t H, int64_t D, const Tensor& 
 void attn_fwd(Tensor q, OptT k, OptT v, Tensor idx, OptT etype, OptT gate, OptT bias, std::vector<Tensor> plan, OptT row_map,
               Tensor acc, Tensor l, OptT m, OptT scratch, int64_t H, int64_t D, int64_t score, int64_t norm, double scale, double lo,
               double hi, int64_t acc_stride, int64_t l_stride, bool accumulate, OptT k_peers, OptT v_peers, int64_t rows_per_peer,
-              int64_t ldq, int64_t ldk, std::vector<int64_t> push_ptrs, int64_t push_rows, int64_t push_ld, int64_t push_l_off) {
+              int64_t ldq, int64_t ldk, std::vector<int64_t> push_ptrs, int64_t push_rows, int64_t push_ld, int64_t push_l_off, OptT o, double eps) {
     c10::cuda::CUDAGuard guard(q.device());
     TORCH_CHECK(q.is_cuda(), "q must be a CUDA tensor");
     if (ldq == 0) check_cuda_contig(q, "q");
@@ -85,7 +85,13 @@ void attn_fwd(Tensor q, OptT k, OptT v, Tensor idx, OptT etype, OptT gate, OptT 
     a.rows_per_peer = (int)rows_per_peer;
     TORCH_CHECK(a.k_peers != nullptr || (a.k != nullptr && a.v != nullptr), "k / v or their peer tables are required");
     a.row_map = cptr<int>(row_map);
-    a.acc = a.push_n > 0 ? nullptr : acc.data_ptr<float>(); a.l = a.push_n > 0 ? nullptr : l.data_ptr<float>();
+    if (o.has_value() && o->defined()) {                 // normalised output in the operand type; `acc` is unused
+        TORCH_CHECK(a.push_n == 0 && !accumulate && a.row_map == nullptr && o->is_contiguous() && o->scalar_type() == q.scalar_type() &&
+                        o->numel() == q.size(0) * H * D && l_stride == H, "normalised output: dense rows of the operand type, no row map, no accumulation");
+        a.o = o->data_ptr();
+        a.eps = (float)eps;
+    }
+    a.acc = (a.push_n > 0 || a.o) ? nullptr : acc.data_ptr<float>(); a.l = a.push_n > 0 ? nullptr : l.data_ptr<float>();
     a.m = m.has_value() && m->defined() ? m->data_ptr<float>() : nullptr;
     a.acc_stride = acc_stride; a.l_stride = l_stride; a.accumulate = accumulate ? 1 : 0;
     gt::attn_fwd(a, stream());
@@ -511,6 +517,19 @@ void pull_unpack(std::vector<int64_t> src_ptrs, int64_t rows_per_peer, int64_t W
                     status.data_ptr<int>(), stream());
 }
 
+void attn_bwd_stat(Tensor dout, Tensor o, Tensor l, OptT m, Tensor stat, bool softmax, double eps) {
+    c10::cuda::CUDAGuard guard(dout.device());
+    TORCH_CHECK(dout.dim() == 3 && dout.scalar_type() == o.scalar_type() && dout.is_contiguous() && o.is_contiguous() && l.is_contiguous() && stat.is_contiguous(),
+                "dout / o [n, H, D] of one dtype, dense l [n, H] and stat [n, H, 4]");
+    TORCH_CHECK(l.scalar_type() == torch::kFloat32 && stat.scalar_type() == torch::kFloat32 && o.numel() == dout.numel() && l.numel() == dout.size(0) * dout.size(1) &&
+                    stat.numel() == 4 * l.numel(), "row statistics");
+    TORCH_CHECK(!m.has_value() || !m->defined() || (m->is_contiguous() && m->scalar_type() == torch::kFloat32 && m->numel() == l.numel()), "m [n, H]");
+    const int H = (int)dout.size(1), D = (int)dout.size(2);
+    TORCH_CHECK(D % 8 == 0 && (D & (D - 1)) == 0 && D <= 256, "head dim must be a power of two from 8 to 256");
+    gt::attn_bwd_stat(dt(dout), dout.data_ptr(), o.data_ptr(), l.data_ptr<float>(), cptr<float>(m), stat.data_ptr(), dout.size(0) * H, D, softmax,
+                      (float)eps, stream());
+}
+
 void attn_bwd_prep(Tensor dacc, Tensor dl, Tensor row_vec, Tensor stat) {
     c10::cuda::CUDAGuard guard(dacc.device());
     TORCH_CHECK(dacc.is_contiguous() && dl.is_contiguous() && row_vec.is_contiguous() && stat.is_contiguous() && dacc.scalar_type() == torch::kFloat32 &&
@@ -691,6 +710,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("sum_payload", &sum_payload);
     m.def("pull_unpack", &pull_unpack);
     m.def("attn_bwd_prep", &attn_bwd_prep);
+    m.def("attn_bwd_stat", &attn_bwd_stat);
     m.def("sum_slots_wait", &sum_slots_wait);
     m.def("allreduce_two_shot", &allreduce_two_shot);
     m.def("channel_wait", &channel_wait);

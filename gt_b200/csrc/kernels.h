@@ -99,6 +99,9 @@ void attn_fwd(const AttnFwdArgs& a, cudaStream_t s);
 void attn_bwd_row(const AttnBwdRowArgs& a, cudaStream_t s);
 void attn_bwd_col(const AttnBwdColArgs& a, cudaStream_t s);
 bool attn_shape_supported(int H, int D, int T);
+// row statistics of the normalised backward: stat[r, h] = {m, -sum_d dout o, 1 / (l or l + eps), 0} for `rows` = n * H heads of D features
+void attn_bwd_stat(int dtype, const void* dout, const void* o, const float* l, const float* m, void* stat, long long rows, int D, bool softmax, float eps,
+                   cudaStream_t s);
 
 // Dense tiles of a block-sparse mask on the tensor cores (attn_tile.cu): adds the tiles' contribution to partial results.
 struct AttnTileArgs {

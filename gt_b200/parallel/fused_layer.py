@@ -183,7 +183,7 @@ class _FusedBranch(torch.autograd.Function):
             acc = torch.empty(rows, hd, dtype=torch.float32, device=dev)
             l = torch.empty(rows, h, dtype=torch.float32, device=dev)
             e.attn_fwd(q_v, k_v, v_v, blk.col, blk.etype, gate_c, None, _plan_list(plan), None, acc, l, None, scratch, h, dh, sc, nm, scale,
-                       lo, hi, hd, h, False, None, None, 0, ldq, ldk, [], 0, 0, 0)
+                       lo, hi, hd, h, False, None, None, 0, ldq, ldk, [], 0, 0, 0, None, 0.0)
             agg = None
             if with_gcn:
                 agg = torch.empty(rows, d, dtype=torch.bfloat16, device=dev)
@@ -195,7 +195,7 @@ class _FusedBranch(torch.autograd.Function):
             mine = [comm.heap.peer_base[r] + poff + comm.row.me * slot_bytes for r in comm.row.ranks]
             dummy = native.status(dev)                      # acc / l are unused when the rows are pushed
             e.attn_fwd(q_v, k_v, v_v, blk.col, blk.etype, gate_c, None, _plan_list(plan), None, dummy, dummy, None, scratch, h, dh, sc, nm,
-                       scale, lo, hi, hd, h, False, None, None, 0, ldq, ldk, mine, o, width, hd)
+                       scale, lo, hi, hd, h, False, None, None, 0, ldq, ldk, mine, o, width, hd, None, 0.0)
             if with_gcn:
                 e.spmm(gm.crow, gm.col, gm.weight, msg_v, dummy, False, _plan_list(gplan), gscratch, [p + (hd + hp) * 2 for p in mine], o, width,
                        rows)
