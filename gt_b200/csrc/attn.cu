@@ -815,20 +815,31 @@ __global__ void attn_bwd_stat_kernel(const T* __restrict__ dout, const T* __rest
     }
 }
 
-// out[i] = sum_b part[b, i]: a block owns 32 columns, its 8 thread rows stride over the partial blocks (coalesced
-// 128-byte reads), the 8 sums are folded through shared memory in a fixed order (deterministic)
-__global__ void reduce_partials_kernel(const float* part, int n_blocks, int width, float* out, int accumulate) {
-    __shared__ float sm[8][33];
+// out[i] = sum_b part[b, i]: a block owns 32 columns, its thread rows stride over the partial blocks (coalesced 128-byte reads), the
+// sums are folded through shared memory in a fixed order (deterministic).  Bound by the latency of a thread row's chain of loads (up to
+// 1776 partial blocks): 32 thread rows with eight loads in flight each.  Eight rows with one load at a time took 21 us for 1776 x 768.
+constexpr int kFoldRows = 32;
+__global__ void __launch_bounds__(32 * kFoldRows) reduce_partials_kernel(const float* __restrict__ part, int n_blocks, int width, float* out, int accumulate) {
+    __shared__ float sm[kFoldRows][33];
     const int i = blockIdx.x * 32 + threadIdx.x;
     float v = 0.f;
-    if (i < width)
-        for (int b = threadIdx.y; b < n_blocks; b += 8) v += part[(size_t)b * width + i];
+    if (i < width) {
+        int b = threadIdx.y;
+        for (; b + 7 * kFoldRows < n_blocks; b += 8 * kFoldRows) {
+            float t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] = __ldg(part + (size_t)(b + k * kFoldRows) * width + i);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v += t[k];
+        }
+        for (; b < n_blocks; b += kFoldRows) v += __ldg(part + (size_t)b * width + i);
+    }
     sm[threadIdx.y][threadIdx.x] = v;
     __syncthreads();
     if (threadIdx.y == 0 && i < width) {
         float t = 0.f;
 #pragma unroll
-        for (int y = 0; y < 8; ++y) t += sm[y][threadIdx.x];
+        for (int y = 0; y < kFoldRows; ++y) t += sm[y][threadIdx.x];
         out[i] = accumulate ? out[i] + t : t;
     }
 }
@@ -1013,7 +1024,7 @@ std::vector<KernelInfo> attn_kernel_info() {
 
 void reduce_partials(const float* part, int n_blocks, int width, float* out, cudaStream_t s, int accumulate) {
     if (width <= 0) return;
-    reduce_partials_kernel<<<(width + 31) / 32, dim3(32, 8), 0, s>>>(part, n_blocks, width, out, accumulate);
+    reduce_partials_kernel<<<(width + 31) / 32, dim3(32, kFoldRows), 0, s>>>(part, n_blocks, width, out, accumulate);
 }
 
 }  // namespace gt

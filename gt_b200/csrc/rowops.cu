@@ -913,32 +913,43 @@ __global__ void bias_act_dropout_bwd_kernel(const T* dout, const T* in, const fl
         for (int i = threadIdx.x; i < d; i += blockDim.x) dbias_part[(size_t)blockIdx.x * d + i] = s_db[i];
 }
 
+// Bound by the rows' reads and writes (2 x 14 MB for 169 K rows of 40 bf16 classes, 4 us) and, as a block per four rows with one atomic on
+// the loss per row, by 92 K atomics on one address: 143 us.  Blocks walk many rows and add their share of the loss once.
 template <typename T>
 __global__ void __launch_bounds__(kWarps * 32) ce_kernel(const T* logits, const long long* labels, const bool* mask, int n, int c,
                                                          float inv_denom, float* loss, T* dlogits) {
-    const int row = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (row >= n) return;
-    const int lane = threadIdx.x & 31;
-    const T* lg = logits + (size_t)row * c;
-    T* dl = dlogits ? dlogits + (size_t)row * c : nullptr;
-    if (!mask[row]) {
-        if (dl) for (int j = lane; j < c; j += 32) dl[j] = from_float<T>(0.f);
-        return;
-    }
-    float mx = -INFINITY;
-    for (int j = lane; j < c; j += 32) mx = fmaxf(mx, to_float(lg[j]));
-    mx = warp_max(mx);
-    float se = 0.f;
-    for (int j = lane; j < c; j += 32) se += __expf(to_float(lg[j]) - mx);
-    se = warp_sum(se);
-    const int y = (int)labels[row];
-    const float lse = mx + __logf(se);
-    if (lane == 0) atomicAdd(loss, (lse - to_float(lg[y])) * inv_denom);
-    if (dl)
-        for (int j = lane; j < c; j += 32) {
-            float pj = __expf(to_float(lg[j]) - lse);
-            dl[j] = from_float<T>((pj - (j == y ? 1.f : 0.f)) * inv_denom);
+    __shared__ float part[kWarps];
+    const int lane = threadIdx.x & 31, wrp = threadIdx.x >> 5;
+    float mine = 0.f;
+    for (int row = blockIdx.x * kWarps + wrp; row < n; row += gridDim.x * kWarps) {
+        const T* lg = logits + (size_t)row * c;
+        T* dl = dlogits ? dlogits + (size_t)row * c : nullptr;
+        if (!mask[row]) {
+            if (dl) for (int j = lane; j < c; j += 32) dl[j] = from_float<T>(0.f);
+            continue;
         }
+        float mx = -INFINITY;
+        for (int j = lane; j < c; j += 32) mx = fmaxf(mx, to_float(lg[j]));
+        mx = warp_max(mx);
+        float se = 0.f;
+        for (int j = lane; j < c; j += 32) se += __expf(to_float(lg[j]) - mx);
+        se = warp_sum(se);
+        const int y = (int)labels[row];
+        const float lse = mx + __logf(se);
+        mine += (lse - to_float(lg[y])) * inv_denom;
+        if (dl)
+            for (int j = lane; j < c; j += 32) {
+                float pj = __expf(to_float(lg[j]) - lse);
+                dl[j] = from_float<T>((pj - (j == y ? 1.f : 0.f)) * inv_denom);
+            }
+    }
+    if (lane == 0) part[wrp] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.f;
+        for (int w = 0; w < kWarps; ++w) t += part[w];
+        atomicAdd(loss, t);
+    }
 }
 
 __global__ void adamw_kernel(AdamWArgs a) {
@@ -1180,7 +1191,7 @@ void bias_act_dropout_bwd(int dtype, const void* dout, const void* in, const flo
 void cross_entropy_fwd_bwd(int dtype, const void* logits, const long long* labels, const bool* mask, int n, int c, float inv_denom,
                            float* loss, void* dlogits, cudaStream_t s) {
     if (n <= 0) return;
-    const int blocks = (n + kWarps - 1) / kWarps;
+    const int blocks = n < 148 * 16 * kWarps ? (n + kWarps - 1) / kWarps : 148 * 16;
     if (dtype == DT_BF16)
         ce_kernel<__nv_bfloat16><<<blocks, kWarps * 32, 0, s>>>(static_cast<const __nv_bfloat16*>(logits), labels, mask, n, c, inv_denom,
                                                                 loss, static_cast<__nv_bfloat16*>(dlogits));
