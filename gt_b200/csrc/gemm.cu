@@ -233,18 +233,26 @@ __global__ void __launch_bounds__(kThreads) gemm_nt_kernel(const __grid_constant
 
 // ------------------------------------------------------------------------------------------------------------------
 // Persistent variant of C = A * B^T.  One CTA per SM walks the output tiles (n fastest, so CTAs running at the same time share
-// the A rows in L2).  Tensor memory holds TWO accumulators (2 x 128 columns): while the epilogue warps drain tile i, the MMA
-// thread already accumulates tile i + 1, and the TMA producer runs ahead through a 5-stage ring that is shared by all tiles
+// the A rows in L2).  Tensor memory holds TWO accumulators (2 x 128 or 2 x 256 columns): while the epilogue warps drain tile i, the MMA
+// thread already accumulates tile i + 1, and the TMA producer runs ahead through a ring that is shared by all tiles
 // (stage indices and phases continue across tile boundaries).  TMEM allocation, barrier initialisation and pipeline fill are
 // paid once per CTA instead of once per tile, which is what bounds the short-K (128..512) GEMMs of these models.
+// The epilogue has two groups of four warps, one per accumulator: a group needs 2 us for a tile (tensor-memory loads, bias /
+// activation / dropout, conversion, staging, stores) while the MMAs of a tile with K = 256 take 0.6 us, so with one group the
+// epilogue set the time of every shape.  The four products of a 256 -> 512 -> 256 feed-forward block over 169 K rows (forward with
+// bias / ReLU, input gradients; 0.16 ms at the copy rate): one group 0.299 ms, a group per accumulator 0.271, with 128 x 256 tiles
+// (gemm_wide) 0.235.
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int P_STAGES = 5;
+constexpr int kEpiGroups = 2, kThreadsP = 64 + kEpiGroups * 128;
+// ring stages that fit next to the staging rows: 4 x 32 KB (columns 128) or 3 x 48 KB (columns 256)
+template <int TBN> struct PersistentShape { static constexpr int kStages = TBN == 128 ? 4 : 3; };
 constexpr int kStageStrideP = BN * 2 + 16;               // staged C row: +16 bytes keeps 16-byte writes conflict-free
 
-struct __align__(1024) PersistentStorage {
+template <int TBN, int P_STAGES = PersistentShape<TBN>::kStages>
+struct __align__(1024) PersistentStorageT {
     __nv_bfloat16 a[P_STAGES][BM * BK];
-    __nv_bfloat16 b[P_STAGES][BN * BK];
-    uint8_t stage_c[4 * 32 * kStageStrideP];
+    __nv_bfloat16 b[P_STAGES][TBN * BK];
+    uint8_t stage_c[kEpiGroups * 4 * 32 * kStageStrideP];
     uint64_t full[P_STAGES];
     uint64_t empty[P_STAGES];
     uint64_t tmem_full[2];
@@ -252,14 +260,19 @@ struct __align__(1024) PersistentStorage {
     uint32_t tmem_base;
     int abort_flag;
 };
+using PersistentStorage = PersistentStorageT<128>;       // of the scatter kernel
+constexpr int P_STAGES = PersistentShape<128>::kStages;
 
-
-__global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
+template <int TBN>
+__global__ void __launch_bounds__(kThreadsP, 1) gemm_nt_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                          const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
     extern __shared__ uint8_t smem_raw[];
-    PersistentStorage& sh = *reinterpret_cast<PersistentStorage*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    using Storage = PersistentStorageT<TBN>;
+    constexpr int P_STAGES = PersistentShape<TBN>::kStages;
+    constexpr bool kSplit = TBN == 256;      // both epilogue groups on every tile, 128 columns each; else a group per accumulator
+    Storage& sh = *reinterpret_cast<Storage*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_n = (g.N + BN - 1) / BN, tiles_m = (g.M + BM - 1) / BM;
+    const int tiles_n = (g.N + TBN - 1) / TBN, tiles_m = (g.M + BM - 1) / BM;
     const int n_tiles = tiles_n * tiles_m;
     const int nkb = (g.K + BK - 1) / BK;
     volatile int* abort_flag = &sh.abort_flag;
@@ -267,10 +280,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
     if (threadIdx.x == 0) {
         sh.abort_flag = 0;
         for (int s = 0; s < P_STAGES; ++s) { mbar_init(&sh.full[s], 1); mbar_init(&sh.empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&sh.tmem_full[b], 1); mbar_init(&sh.tmem_empty[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&sh.tmem_full[b], 1); mbar_init(&sh.tmem_empty[b], kSplit ? 8 : 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(&sh.tmem_base, 2 * kTmemCols);
+    if (warp == 1) tmem_alloc(&sh.tmem_base, 2 * TBN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -281,12 +294,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
         int it = 0, issued_from = 0;
         bool okay = true;
         for (int tile = blockIdx.x; tile < n_tiles && okay; tile += gridDim.x) {
-            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * TBN;
             for (int kb = 0; kb < nkb; ++kb, ++it) {
                 const int s = it % P_STAGES;
                 okay = mbar_wait(&sh.empty[s], ((it / P_STAGES) & 1) ^ 1, abort_flag, g.status, 1);
                 if (!okay) break;
-                mbar_expect_tx(&sh.full[s], (BM + BN) * BK * 2);
+                mbar_expect_tx(&sh.full[s], (BM + TBN) * BK * 2);
                 tma_load_2d(sh.a[s], &map_a, kb * BK, m0, &sh.full[s]);
                 tma_load_2d(sh.b[s], &map_b, kb * BK, n0, &sh.full[s]);
             }
@@ -301,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
         }
     } else if (warp == 1 && lane == 0) {
         // ---- MMA issuer ----
-        const uint32_t idesc = make_idesc(BM, BN, 0, 0);
+        const uint32_t idesc = make_idesc(BM, TBN, 0, 0);
         int it = 0, ti = 0;
         bool okay = true;
         for (int tile = blockIdx.x; tile < n_tiles && okay; tile += gridDim.x, ++ti) {
@@ -309,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
             okay = mbar_wait(&sh.tmem_empty[b], ((ti >> 1) & 1) ^ 1, abort_flag, g.status, 2);   // epilogue drained this accumulator
             if (!okay) break;
             tc_fence_after();
-            const uint32_t acc = tmem + (uint32_t)(b * BN);
+            const uint32_t acc = tmem + (uint32_t)(b * TBN);
             for (int kb = 0; kb < nkb; ++kb, ++it) {
                 const int s = it % P_STAGES;
                 okay = mbar_wait(&sh.full[s], (it / P_STAGES) & 1, abort_flag, g.status, 2);
@@ -325,19 +338,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
         }
     } else if (warp >= 2) {
         // ---- epilogue ----
-        const int quad = warp & 3;
+        const int quad = warp & 3, grp = (warp - 2) >> 2;         // see kSplit
         const uint64_t sd = site_seed(g.seed, g.stream_id);
         const float inv_keep = g.p > 0.f ? keep_scale(g.p) : 1.f;
         const bool staged = g.c_dtype == DT_BF16 && (g.ldc & 7) == 0 && (g.N & 7) == 0;
-        uint8_t* stage = sh.stage_c + (size_t)quad * 32 * kStageStrideP;
-        int ti = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++ti) {
+        uint8_t* stage = sh.stage_c + (size_t)(grp * 4 + quad) * 32 * kStageStrideP;
+        constexpr int kStep = kSplit ? 1 : kEpiGroups;
+        const int coff = kSplit ? grp * 128 : 0;
+        int ti = kSplit ? 0 : grp;
+        for (int tile = blockIdx.x + ti * gridDim.x; tile < n_tiles; tile += kStep * gridDim.x, ti += kStep) {
             const int b = ti & 1;
-            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * BN;
+            const int m0 = (tile / tiles_n) * BM, n0 = (tile % tiles_n) * TBN + coff;
             if (!mbar_wait(&sh.tmem_full[b], (ti >> 1) & 1, abort_flag, g.status, 3)) break;
             tc_fence_after();
             const int row = m0 + quad * 32 + lane;
-            const uint32_t acc = tmem + (uint32_t)(b * BN) + ((uint32_t)(quad * 32) << 16);
+            const uint32_t acc = tmem + (uint32_t)(b * TBN + coff) + ((uint32_t)(quad * 32) << 16);
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t r[32];
                 __syncwarp();                                 // lanes that skipped the previous chunk rejoin before the aligned load
@@ -399,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nt_persistent_kernel(const _
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 2 * kTmemCols);
+    if (warp == 1) tmem_dealloc(tmem, 2 * TBN);
 }
 
 // ------------------------------------------------------------------------------------------------------------------
@@ -1120,11 +1135,19 @@ static char env_kernel() {
     return env ? env[0] : 0;
 }
 
+// 128 x 256 tiles re-read A half as often and take 192 KB instead of 256 KB of operands per 256 columns and K = 256 (0.271 -> 0.235 ms
+// over the products named above, 0.128 -> 0.107 ms for 512 -> 1024 -> 512 over 20 K rows).  They need whole tiles, and two rounds of
+// them: below that the finer 128-column tiles spread over more SMs.
+static bool gemm_wide(const GemmArgs& g) {
+    return g.N % 256 == 0 && (long long)(g.N / 256) * ((g.M + BM - 1) / BM) >= 2 * 148;
+}
+
 int gemm_tcgen05(const GemmArgs& g, cudaStream_t s) {
     if ((reinterpret_cast<uintptr_t>(g.a) & 15) || (reinterpret_cast<uintptr_t>(g.b) & 15)) return -2;
     CUtensorMap ma, mb;
     if (!make_map(&ma, g.a, g.M, g.K, g.lda, BM, BK)) return -1;
-    if (!make_map(&mb, g.b, g.N, g.K, g.ldb, BN, BK)) return -1;
+    const bool wide = gemm_wide(g);
+    if (!make_map(&mb, g.b, g.N, g.K, g.ldb, wide ? 256 : BN, BK)) return -1;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(gemm_nt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
@@ -1138,7 +1161,8 @@ int gemm_tcgen05(const GemmArgs& g, cudaStream_t s) {
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
         const char* env = getenv("GT_GEMM_KERNEL");
         simple = env && env[0] == 's';                    // "simple": the one-tile-per-CTA kernel (comparison / debugging)
-        cudaFuncSetAttribute(gemm_nt_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(PersistentStorage) + 1024));
+        cudaFuncSetAttribute(gemm_nt_persistent_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(PersistentStorageT<128>) + 1024));
+        cudaFuncSetAttribute(gemm_nt_persistent_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(PersistentStorageT<256>) + 1024));
     }
     // GT_GEMM_KERNEL=a: run local short-K products on the A-stationary kernel of the fused all-gather (one "peer": this GPU).
     // Measured on 169,344 x 256 -> 1024 / 512 / 256 and 512 -> 256: the tile-walking kernel is faster on every shape (0.142 /
@@ -1150,11 +1174,14 @@ int gemm_tcgen05(const GemmArgs& g, cudaStream_t s) {
         return gemm_nt_gather(g, self, 1, g.M, nullptr, s, nullptr);
     }
     if (simple) {
+        if (wide && !make_map(&mb, g.b, g.N, g.K, g.ldb, BN, BK)) return -1;
         dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM);
         gemm_nt_kernel<<<grid, kThreads, kSmemBytes, s>>>(ma, mb, g);
     } else {
-        const int tiles = ((g.N + BN - 1) / BN) * ((g.M + BM - 1) / BM);
-        gemm_nt_persistent_kernel<<<tiles < n_sm ? tiles : n_sm, kThreads, sizeof(PersistentStorage) + 1024, s>>>(ma, mb, g);
+        const int tbn = wide ? 256 : BN;
+        const int tiles = ((g.N + tbn - 1) / tbn) * ((g.M + BM - 1) / BM), grid = tiles < n_sm ? tiles : n_sm;
+        if (wide) gemm_nt_persistent_kernel<256><<<grid, kThreadsP, sizeof(PersistentStorageT<256>) + 1024, s>>>(ma, mb, g);
+        else gemm_nt_persistent_kernel<128><<<grid, kThreadsP, sizeof(PersistentStorageT<128>) + 1024, s>>>(ma, mb, g);
     }
     return (int)cudaGetLastError();
 }
