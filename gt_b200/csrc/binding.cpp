@@ -298,7 +298,7 @@ void premp_bwd(Tensor h, Tensor dout, Tensor gamma, Tensor beta, Tensor stats, T
     gt::premp(a, true, stream());
 }
 
-int64_t layer_norm_bwd_blocks(int64_t n) { return gt::layer_norm_bwd_blocks((int)n); }
+int64_t layer_norm_bwd_blocks(int64_t n, bool bf16, int64_t d) { return gt::layer_norm_bwd_blocks((int)n, bf16 ? gt::DT_BF16 : gt::DT_F32, (int)d); }
 
 void layer_norm_bwd(Tensor dout, Tensor y, OptT x, OptT ybias, Tensor gamma, Tensor mean_rstd, Tensor dy, OptT dx, bool accumulate_dx,
                     Tensor dgamma_part, Tensor dbeta_part, OptT dybias_part, double p, OptT seed, int64_t stream_id, OptT acc, OptT l,

@@ -205,7 +205,7 @@ struct LayerNormBwdArgs {
     const float* acc; const float* l; int H; float eps_l; float* dacc; float* dl;
 };
 void layer_norm_bwd(const LayerNormBwdArgs& a, cudaStream_t s);
-int layer_norm_bwd_blocks(int n);
+int layer_norm_bwd_blocks(int n, int dtype, int d);
 
 // elementwise epilogue used when a GEMM is not fused: out = drop(act(in + bias))
 void bias_act_dropout(int dtype, const void* in, const float* bias, void* out, long long n, int d, int act, float p,

@@ -259,11 +259,16 @@ __global__ void __launch_bounds__(kWarps * 32) ln_bwd_kernel(LayerNormBwdArgs a)
 
 // ------------------------------------------------------------------------------------------------------------------
 // LayerNorm kernels for rows of up to 256 bf16 features whose operands arrive through a per-thread cp.async ring in shared
-// memory: a warp keeps the loads of kLnStages - 1 future rows in flight without holding them in registers (a row is a
+// memory: a warp keeps the loads of the next rows in flight without holding them in registers (a row is a
 // dependent chain of load -> two warp reductions -> store, so bandwidth comes only from rows in flight).  Every lane copies and
 // later reads only its own chunks: no synchronisation between lanes.  Same arithmetic as ln_fwd_kernel / ln_bwd_kernel.
+//
+// A row keeps its warp in two dependent warp reductions and about 280 (forward) or 450 (backward) instructions, so it is warps per SM
+// and not rows in flight per warp that count: with eight stages a block took 61 to 78 KB and two or three were resident.  Three or four
+// stages let eight (forward) or four (backward: 128 registers) run, and the backward runs one resident wave (its blocks fold 24 sums per
+// lane at the end).  169 K rows x 256, fp32 attention accumulator / bf16 branch output: forward 89 -> 65 / 66 -> 66 us, backward
+// 169 -> 106 / 108 -> 80 us (floors 52 / 39 and 91 / 65).
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int kLnStages = 8;
 
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gsrc) : "memory");
@@ -284,28 +289,29 @@ __device__ __forceinline__ void unpack_bf16x8(const uint4& u, float (&f)[8]) {
 template <bool ACC, bool BWD>
 struct LnRing {
     static constexpr int kSlots = (ACC ? 2 : 1) + 1 + (BWD ? 1 : 0);            // y (or acc lo / hi), x, dout
+    static constexpr int kStages = ACC && !BWD ? 3 : 4;                         // what lets 8 (forward) or 4 (backward) blocks share an SM
     static constexpr int kThreads = kWarps * 32;
-    static constexpr size_t kBytes = (size_t)kLnStages * kThreads * (kSlots * 16 + 8 + 4);
+    static constexpr size_t kBytes = (size_t)kStages * kThreads * (kSlots * 16 + 8 + 4);
     uint4* data; float2* stat; float* lv;
     __device__ LnRing(uint8_t* base) {
         data = reinterpret_cast<uint4*>(base);
-        stat = reinterpret_cast<float2*>(base + (size_t)kLnStages * kThreads * kSlots * 16);
-        lv = reinterpret_cast<float*>(base + (size_t)kLnStages * kThreads * (kSlots * 16 + 8));
+        stat = reinterpret_cast<float2*>(base + (size_t)kStages * kThreads * kSlots * 16);
+        lv = reinterpret_cast<float*>(base + (size_t)kStages * kThreads * (kSlots * 16 + 8));
     }
     __device__ uint4* slot(int stage, int s) const { return data + ((size_t)stage * kSlots + s) * kThreads + threadIdx.x; }
 };
 
 template <bool ACC>
-__global__ void __launch_bounds__(kWarps * 32) ln_fwd_ring_kernel(LayerNormArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, 8) ln_fwd_ring_kernel(LayerNormArgs a) {
     extern __shared__ __align__(16) uint8_t ring_raw[];
     using Ring = LnRing<ACC, false>;
     Ring ring(ring_raw);
-    constexpr int NS = kLnStages, SX = ACC ? 2 : 1;
+    constexpr int NS = Ring::kStages, SX = ACC ? 2 : 1;
     const int lane = threadIdx.x & 31, nch = a.d >> 3, f = lane << 3;
     const bool active = lane < nch;
     const uint64_t sd = site_seed(a.seed, a.stream_id);
     const float inv_keep = a.p > 0.f ? keep_scale(a.p) : 1.f;
-    const int hd = ACC ? a.d / a.H : a.d;
+    const int hd = ACC ? a.d / a.H : a.d, head = ACC ? f / hd : 0;
     const __nv_bfloat16* yb16 = static_cast<const __nv_bfloat16*>(a.y);
     const __nv_bfloat16* xb16 = static_cast<const __nv_bfloat16*>(a.x);
     float gam[8], bet[8], ybv[8];
@@ -317,28 +323,29 @@ __global__ void __launch_bounds__(kWarps * 32) ln_fwd_ring_kernel(LayerNormArgs 
     }
     const int n_warps = gridDim.x * kWarps, w = blockIdx.x * kWarps + (threadIdx.x >> 5);
     const int n_k = w < a.n ? (a.n - w + n_warps - 1) / n_warps : 0;
+    int fill = 0, st = 0;                               // ring stages of the next row to fetch and of the current row
     auto issue = [&](int k) {
         if (k < n_k && active) {
             const size_t row = (size_t)w + (size_t)k * n_warps;
-            const int st = k % NS;
+            const int st = fill;
             if (ACC) {
                 cp_async_16(ring.slot(st, 0), a.acc + row * a.d + f);
                 cp_async_16(ring.slot(st, 1), a.acc + row * a.d + f + 4);
-                cp_async_4(ring.lv + st * Ring::kThreads + threadIdx.x, a.l + row * a.H + f / hd);
+                cp_async_4(ring.lv + st * Ring::kThreads + threadIdx.x, a.l + row * a.H + head);
             } else {
                 cp_async_16(ring.slot(st, 0), yb16 + row * a.d + f);
             }
             if (a.x) cp_async_16(ring.slot(st, SX), xb16 + row * a.d + f);
         }
+        if (++fill == NS) fill = 0;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
     for (int k = 0; k < NS - 1; ++k) issue(k);
-    for (int k = 0; k < n_k; ++k) {
+    for (int k = 0; k < n_k; ++k, st = st + 1 == NS ? 0 : st + 1) {
         issue(k + NS - 1);
         asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
         const size_t row = (size_t)w + (size_t)k * n_warps;
-        const int st = k % NS;
         float z[8];
         float sum = 0.f;
         if (active) {
@@ -382,19 +389,19 @@ __global__ void __launch_bounds__(kWarps * 32) ln_fwd_ring_kernel(LayerNormArgs 
 }
 
 template <bool ACC>
-__global__ void __launch_bounds__(kWarps * 32) ln_bwd_ring_kernel(LayerNormBwdArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, 4) ln_bwd_ring_kernel(LayerNormBwdArgs a) {
     extern __shared__ __align__(16) uint8_t ring_raw[];
     using Ring = LnRing<ACC, true>;
     float* acc_sm = reinterpret_cast<float*>(ring_raw);                          // [3][d] block accumulators first, the ring after them
     Ring ring(ring_raw + ((3 * (size_t)a.d * sizeof(float) + 15) & ~size_t(15)));
-    constexpr int NS = kLnStages, SX = ACC ? 2 : 1, SD = SX + 1;
+    constexpr int NS = Ring::kStages, SX = ACC ? 2 : 1, SD = SX + 1;
     const int lane = threadIdx.x & 31, nch = a.d >> 3, f = lane << 3;
     const bool active = lane < nch;
     for (int i = threadIdx.x; i < 3 * a.d; i += blockDim.x) acc_sm[i] = 0.f;
     __syncthreads();
     const uint64_t sd = site_seed(a.seed, a.stream_id);
     const float inv_keep = a.p > 0.f ? keep_scale(a.p) : 1.f;
-    const int hd = ACC ? a.d / a.H : a.d;
+    const int hd = ACC ? a.d / a.H : a.d, head = ACC ? f / hd : 0;
     const __nv_bfloat16* yb16 = static_cast<const __nv_bfloat16*>(a.y);
     const __nv_bfloat16* xb16 = static_cast<const __nv_bfloat16*>(a.x);
     const __nv_bfloat16* gob16 = static_cast<const __nv_bfloat16*>(a.dout);
@@ -407,14 +414,15 @@ __global__ void __launch_bounds__(kWarps * 32) ln_bwd_ring_kernel(LayerNormBwdAr
     }
     const int n_warps = gridDim.x * kWarps, w = blockIdx.x * kWarps + (threadIdx.x >> 5);
     const int n_k = w < a.n ? (a.n - w + n_warps - 1) / n_warps : 0;
+    int fill = 0, st = 0;                               // ring stages of the next row to fetch and of the current row
     auto issue = [&](int k) {
         if (k < n_k && active) {
             const size_t row = (size_t)w + (size_t)k * n_warps;
-            const int st = k % NS;
+            const int st = fill;
             if (ACC) {
                 cp_async_16(ring.slot(st, 0), a.acc + row * a.d + f);
                 cp_async_16(ring.slot(st, 1), a.acc + row * a.d + f + 4);
-                cp_async_4(ring.lv + st * Ring::kThreads + threadIdx.x, a.l + row * a.H + f / hd);
+                cp_async_4(ring.lv + st * Ring::kThreads + threadIdx.x, a.l + row * a.H + head);
             } else {
                 cp_async_16(ring.slot(st, 0), yb16 + row * a.d + f);
             }
@@ -422,15 +430,15 @@ __global__ void __launch_bounds__(kWarps * 32) ln_bwd_ring_kernel(LayerNormBwdAr
             cp_async_16(ring.slot(st, SD), gob16 + row * a.d + f);
             cp_async_8(ring.stat + st * Ring::kThreads + threadIdx.x, a.mean_rstd + 2 * row);
         }
+        if (++fill == NS) fill = 0;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
     for (int k = 0; k < NS - 1; ++k) issue(k);
-    for (int k = 0; k < n_k; ++k) {
+    for (int k = 0; k < n_k; ++k, st = st + 1 == NS ? 0 : st + 1) {
         issue(k + NS - 1);
         asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
         const size_t row = (size_t)w + (size_t)k * n_warps;
-        const int st = k % NS;
         float zh[8], dzh[8], av[8];
         uint32_t keep_bits = 0u;
         float s1 = 0.f, s2 = 0.f, rstd = 0.f, inv_l = 1.f;
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(kWarps * 32) ln_bwd_ring_kernel(LayerNormBwdAr
             const int lph = hd >> 3;
             float v = dl_part;
             for (int o = lph >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(GT_FULL_MASK, v, o);
-            if (active && (lane & (lph - 1)) == 0) a.dl[row * a.H + f / hd] = v;
+            if (active && (lane & (lph - 1)) == 0) a.dl[row * a.H + head] = v;
         }
     }
     if (active) {
@@ -1092,9 +1100,9 @@ void layer_norm_fwd(const LayerNormArgs& a, cudaStream_t s) {
     const bool aligned = (reinterpret_cast<uintptr_t>(a.y) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(a.acc) & 15) == 0;
     if (use_ring && a.dtype == DT_BF16 && a.d <= 256 && aligned) {
-        // operands through the cp.async ring; 5 blocks of 4 warps per SM fit next to their rings
+        // operands through the cp.async ring; 8 blocks of 4 warps per SM
         int rb = (a.n + kWarps - 1) / kWarps;
-        if (rb > 148 * 5) rb = 148 * 5;
+        if (rb > 148 * 8) rb = 148 * 8;
         if (a.acc) {
             static bool once = (cudaFuncSetAttribute(ln_fwd_ring_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LnRing<true, false>::kBytes), true);
             (void)once;
@@ -1118,9 +1126,15 @@ void layer_norm_fwd(const LayerNormArgs& a, cudaStream_t s) {
 #undef GT_LN_FWD
 }
 
-int layer_norm_bwd_blocks(int n) {
-    int b = grid_for(n, kWarps * 8);
-    return b > 148 * 12 ? 148 * 12 : b;                // enough resident warps to hide the row latency
+static bool ln_ring_shape(int dtype, int d) {
+    static const bool use_ring = [] { const char* e = getenv("GT_LN_RING"); return !(e && e[0] == '0'); }();
+    return use_ring && dtype == DT_BF16 && d <= 256;
+}
+
+// ring kernel: one resident wave; register kernels: enough resident warps to hide the row latency
+int layer_norm_bwd_blocks(int n, int dtype, int d) {
+    const int b = grid_for(n, kWarps * 8), cap = ln_ring_shape(dtype, d) ? 148 * 4 : 148 * 12;
+    return b > cap ? cap : b;
 }
 
 void layer_norm_bwd(const LayerNormBwdArgs& a, cudaStream_t s) {

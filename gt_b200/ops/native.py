@@ -318,7 +318,7 @@ class _LayerNorm(torch.autograd.Function):
         n, d = y.shape
         acc_mode = l is not None
         like = x if acc_mode else y
-        nb = e.layer_norm_bwd_blocks(n)
+        nb = e.layer_norm_bwd_blocks(n, like.dtype == torch.bfloat16, d)
         parts = torch.empty(nb, 3, d, dtype=torch.float32, device=y.device)      # the block partials of all three sums side by side
         dy = torch.empty_like(y)                                  # acc mode: this is dacc (fp32)
         dl = torch.empty_like(l) if acc_mode else None
