@@ -3,8 +3,8 @@
 // What bounds them: every edge moves one or two gathered feature rows of up to 512 bytes through the load path and does a few
 // hundred multiply-adds on them, so the limits are the gather traffic and, long before that is reached, the number of warp
 // instructions spent per edge.  The previous kernels (one 16-byte chunk per lane, a cp.async ring in shared memory, every lane of a
-// head repeating the head's softmax arithmetic) issued 98 / 197 / 103 warp instructions per edge in the forward / column / row pass
-// (8 heads of 32, bf16) and ran at 60 % of the issue slots and 20 % of the L2 throughput.  Here:
+// head repeating the head's softmax arithmetic) issued 183 / 95 warp instructions per edge in the column / row pass (8 heads of 32,
+// bf16) and ran at 60 % of the issue slots and 20 % of the L2 throughput.  Here:
 //   * a lane owns 8 consecutive features (16 bytes of bf16); a feature row of up to 256 features is covered by LPR = H*D/8 lanes, a
 //     warp walks one segment with 32 / LPR edges side by side, and 512 features are two independent halves of the heads (grid.y);
 //   * the indices and types of 32 edges are fetched by one coalesced load and handed round by shuffles, the type only matters where it
@@ -15,7 +15,7 @@
 //     score: exponential, clamp, statistics and score gradient are evaluated once per (edge, head) instead of once per lane;
 //   * accumulations are packed pairs (fma.rn.f32x2): half the issue slots for the same fp32 arithmetic.
 // Rows by direct loads into registers (no ring) needed 32 registers a group more and spilled or halved the warps in flight: 0.44 /
-// 1.05 / 0.50 ms against 0.36 / 0.67 / 0.36 ms for the three passes (169 K nodes, 4.03 M edges, 8 heads x 32).  A plain gather of the
+// 1.05 / 0.50 ms against 0.36 / 0.69 / 0.37 ms for the three passes (ring kernels replaced: 0.61 / 1.07 / 0.53) (169 K nodes, 4.03 M edges, 8 heads x 32).  A plain gather of the
 // same rows runs at 12.4 TB/s when the operands are 174 MB (19 TB/s at 87 MB, 8 TB/s at 512 MB, measured with 512-byte rows), which
 // puts the floor of the forward at 0.31 ms.
 // The sums over the features of a head, over the edges of a segment and over the lane groups are taken in the same order as by the
